@@ -103,8 +103,10 @@ def _device_graph(case, seed):
     return device_rmat_graph(v, pairs, seed=seed, device=torch.device(DEVICE))
 
 
-def _graph(case, seed):
-    v, pairs = case["vertices"], case["pairs"]
+def _dataset_graph(case):
+    """The graph of a training case is a data set's: the same one for every seed, as in bench.py and tools/bench_configs.py.
+    Features, labels, masks and initial weights are drawn anew."""
+    v, pairs, seed = case["vertices"], case["pairs"], 1
     if case["graph"] == "er":
         return erdos_renyi(v, 2.0 * pairs / v, seed=seed)
     if case["graph"] == "rmat_directed":
@@ -141,7 +143,7 @@ def prepare(case, seed):
             state["dy"], state["dx"] = _randn(gen, v, w), ops.alloc2d(v, w, DEVICE)
         return state
     v, c = case["vertices"], case["classes"]
-    graph = _graph(case, seed)
+    graph = _dataset_graph(case)
     features = torch.randn(v, case["features"], generator=gen, device=DEVICE)
     labels = torch.zeros(v, c, device=DEVICE)
     labels.scatter_(1, torch.randint(0, c, (v, 1), generator=gen, device=DEVICE), 1.0)
