@@ -361,6 +361,28 @@ def test_adam_and_sgd_tables():
         assert float(tab.hp[5]) == 3.0
 
 
+@pytest.mark.parametrize("splits", [2, 7, 8, 9, 63, 64, 65, 296])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 41), (64, 16), (130, 256)])
+def test_splitk_reduce_sums_every_split(splits, rows, cols):
+    """Ordered sum of split-K partials at the edges of a block (32 groups) and of both slice counts; the padding columns of
+    the result stay as they are.  At most `splits` fp32 additions per element: |error| <= splits * 2^-24 * sum |partial|."""
+    out = ops.alloc2d(rows, cols, DEV)
+    ld = ops.api._ld(out)
+    full = out.as_strided((rows, ld), (ld, 1))
+    gen = torch.Generator().manual_seed(splits)
+    part = torch.randn(splits, rows, ld, generator=gen).to(DEV)
+    for accumulate in (0, 1):
+        full.fill_(3.0)
+        rc = ops.api._k().mk_splitk_reduce(part.data_ptr(), rows * ld, splits, out.data_ptr(), rows, cols, ld, accumulate, ops.api._stream())
+        assert rc == 0
+        ref = part.double().sum(0) + (3.0 if accumulate else 0.0)
+        bound = (splits + 1) * 2.0 ** -24 * (part.double().abs().sum(0) + 3.0)
+        got = full.double()
+        groups = (cols + 3) // 4 * 4
+        assert bool(((got - ref).abs() <= bound)[:, :groups].all())
+        assert bool((full[:, groups:] == 3.0).all())
+
+
 @pytest.mark.parametrize("is_max", [True, False])
 @pytest.mark.parametrize("width", [5, 64, 200])
 def test_extreme_aggregation_matches_oracle(is_max, width):
