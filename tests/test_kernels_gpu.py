@@ -472,3 +472,37 @@ def test_debug_index_validation_kernels(monkeypatch):
     torch.testing.assert_close(out.cpu(), ref, rtol=1e-4, atol=1e-5)
     with pytest.raises(validate.IndexValidationError):
         ops.spmm(NormalizedCSR(a.rowptr, bad_col, a.val, a.num_rows, a.num_cols), x, out)
+
+
+@pytest.mark.parametrize("tiles", [False, True])
+@pytest.mark.parametrize("width", [3, 16, 41, 64, 100, 128, 256, 300])
+def test_spmm_fused_epilogue(tiles, width, request):
+    """Every step of the aggregation's epilogue (factor, mix in front of or behind the ReLU, copy, ReLU mask) on a matrix
+    with split rows, with and without dense tiles (rows that already hold their tile part).  The epilogue is checked
+    against the same steps applied to the plain product in float32: a mismatch beyond rounding is a wrong step."""
+    if tiles:
+        request.getfixturevalue("tiles_on_small_matrices")
+    g = _dense_corner_graph()
+    csr = build_normalized_csr(g).to(DEV)
+    assert (ops.api.tile_plan(csr) is not None) == tiles
+    n = g.num_vertices
+    x, mix, mask = _rand2d(n, width, 1), _rand2d(n, width, 2), _rand2d(n, width, 3)
+    base = ops.alloc2d(n, width, DEV)
+    ops.spmm(csr, x, base)
+    out, plain = ops.alloc2d(n, width, DEV), ops.alloc2d(n, width, DEV)
+    tol = 1e-6 * float(base.abs().max() + mix.abs().max())          # a few roundings of one term
+
+    def close(a, b):
+        return float((a - b).abs().max()) <= tol
+
+    ops.spmm(csr, x, out, alpha=0.9, mix=(mix, 0.1))                              # GCNII's P
+    assert close(out, 0.9 * base + 0.1 * mix)
+    ops.spmm(csr, x, out, relu=True, mix=(mix, 1.0))                              # ADD, then ReLU
+    assert close(out, torch.relu(base + mix))
+    ops.spmm(csr, x, out, relu=True, mix=(mix, 1.0), mix_after_relu=True, plain=plain)      # residual layer
+    assert close(plain, torch.relu(base)) and close(out, torch.relu(base) + mix)
+    ops.spmm(csr, x, out, alpha=0.9, relu_mask=mask)                              # backward through a ReLU
+    assert close(out, 0.9 * base * (mask > 0))
+    ld = ops.api._ld(out)
+    for t in (out, plain):
+        assert float(t.as_strided((n, ld), (ld, 1))[:, width:].abs().sum()) == 0.0
