@@ -540,3 +540,42 @@ def test_spmm_every_row_width_and_number_of_rounds(rows, width):
     assert bool(((out.cpu().double() - torch.relu(ref)).abs() <= bound).all())
     ld = ops.api._ld(out)
     assert float(out.as_strided((rows, ld), (ld, 1))[:, width:].abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("n,k,m", [(1, 1, 1), (127, 33, 17), (128, 32, 128), (129, 31, 129), (300, 64, 160), (1000, 7, 256), (260, 602, 41), (20001, 256, 300)])
+def test_gemm_split3_kernel(n, k, m):
+    """The fp32-accurate tensor-core product at the edges of its tiles (rows, columns, reduction, several column tiles, more
+    tiles than SMs, split reductions), in the three layouts, with factor, mask and accumulation.  Bound per element, against
+    float64: 2^-21 of the sum of absolute products for the split plus one fp32 rounding per eight terms of the reduction."""
+    def run(a, b, out, trans_a=False, trans_b=False, alpha=1.0, accumulate=False, mask=None):
+        M, K = (a.shape[1], a.shape[0]) if trans_a else (a.shape[0], a.shape[1])
+        N = b.shape[0] if trans_b else b.shape[1]
+        ops.api._gemm_split3(a, b, out, trans_a, M, N, K, int(trans_a), 0 if trans_b else 1, alpha, accumulate, mask,
+                             mask.data_ptr() if mask is not None else None)
+
+    def check(out, a, b, alpha, base=None, mask=None):
+        ref, scale = alpha * (a @ b), abs(alpha) * (a.abs() @ b.abs())
+        if mask is not None:
+            ref = ref * (mask > 0)
+        if base is not None:
+            ref, scale = ref + base, scale + base.abs()
+        bound = (2.0 ** -21 + (a.shape[1] / 8 + 4) * 2.0 ** -23) * scale + 1e-30
+        assert bool(((out.cpu().double() - ref).abs() <= bound).all())
+        rows, cols = out.shape
+        ld = ops.api._ld(out)
+        assert rows == 1 or float(out.as_strided((rows, ld), (ld, 1))[:, cols:].abs().sum()) == 0.0
+
+    x, w, dy, mask = _rand2d(n, k, 1), _rand2d(k, m, 2), _rand2d(n, m, 3), _rand2d(n, k, 4)
+    X, W, DY, MASK = (t.cpu().double() for t in (x, w, dy, mask))
+    out = ops.alloc2d(n, m, DEV)
+    run(x, w, out, alpha=0.5)
+    check(out, X, W, 0.5)
+    dx = _rand2d(n, k, 5)
+    base = dx.cpu().double()
+    run(dy, w, dx, trans_b=True, accumulate=True, mask=mask)
+    check(dx, DY, W.t(), 1.0, base, MASK)
+    dw = _rand2d(k, m, 6)
+    base = dw.cpu().double()
+    run(x, dy, dw, trans_a=True, accumulate=True)
+    check(dw, X.t(), DY, 1.0, base)
+    _status_ok()
