@@ -362,11 +362,11 @@ def test_adam_and_sgd_tables():
         assert float(tab.hp[5]) == 3.0
 
 
-@pytest.mark.parametrize("splits", [2, 7, 8, 9, 63, 64, 65, 296])
+@pytest.mark.parametrize("splits", [2, 7, 8, 9, 63, 64, 65, 296, 319, 320, 321, 700])
 @pytest.mark.parametrize("rows,cols", [(1, 1), (3, 41), (64, 16), (130, 256)])
 def test_splitk_reduce_sums_every_split(splits, rows, cols):
-    """Ordered sum of split-K partials at the edges of a block (32 groups) and of both slice counts; the padding columns of
-    the result stay as they are.  At most `splits` fp32 additions per element: |error| <= splits * 2^-24 * sum |partial|."""
+    """Ordered sum of split-K partials at the edges of a block (8 groups) and of its chunks of splits (320); the padding columns
+    of the result stay as they are.  At most `splits` fp32 additions per element: |error| <= splits * 2^-24 * sum |partial|."""
     out = ops.alloc2d(rows, cols, DEV)
     ld = ops.api._ld(out)
     full = out.as_strided((rows, ld), (ld, 1))
