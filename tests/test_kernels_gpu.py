@@ -579,3 +579,19 @@ def test_gemm_split3_kernel(n, k, m):
     run(x, dy, dw, trans_a=True, accumulate=True)
     check(dw, X.t(), DY, 1.0, base)
     _status_ok()
+
+
+@pytest.mark.parametrize("n,k,m", [(63, 5, 3), (64, 64, 64), (127, 65, 7), (129, 1, 1), (1000, 33, 130), (12803, 105, 51), (26416, 25, 4)])
+def test_gemm_fp32_weight_gradient_split_reduction(n, k, m):
+    """Exact-fp32 weight gradients below the tensor-core threshold: the reduction over the vertices is cut into parts.  At most
+    one fp32 rounding per term and per part; padding columns stay zero."""
+    assert n * k * m < 1 << 27
+    x, dy, dw = _rand2d(n, k, 1), _rand2d(n, m, 2), _rand2d(k, m, 3)
+    X, DY, base = x.cpu().double(), dy.cpu().double(), dw.cpu().double()
+    for accumulate in (True, False):
+        ops.gemm(x, dy, dw, trans_a=True, accumulate=accumulate, alpha=0.5, precision="fp32")
+        ref = 0.5 * X.t() @ DY + (base if accumulate else 0.0)
+        bound = (n + 300) * 2.0 ** -24 * (0.5 * X.abs().t() @ DY.abs() + base.abs())
+        assert bool(((dw.cpu().double() - ref).abs() <= bound).all())
+        ld = ops.api._ld(dw)
+        assert k == 1 or float(dw.as_strided((k, ld), (ld, 1))[:, m:].abs().sum()) == 0.0
