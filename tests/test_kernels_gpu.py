@@ -595,3 +595,22 @@ def test_gemm_fp32_weight_gradient_split_reduction(n, k, m):
         assert bool(((dw.cpu().double() - ref).abs() <= bound).all())
         ld = ops.api._ld(dw)
         assert k == 1 or float(dw.as_strided((k, ld), (ld, 1))[:, m:].abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("shapes", [[(1, 4)], [(16, 64)], [(602, 256), (256, 41), (7, 3)], [(2400, 512)]])
+def test_adam_advances_its_step_once_per_launch(shapes):
+    """One block, several, and more work than the grid has threads: the step counter moves by one per launch and the ticket
+    word is back at zero; the weights follow the oracle, whose first bias corrections depend on the counter."""
+    w, g = [_rand2d(r, c, i) for i, (r, c) in enumerate(shapes)], [_rand2d(r, c, 10 + i) for i, (r, c) in enumerate(shapes)]
+    ref, rg = [t.cpu().clone() for t in w], [t.cpu() for t in g]
+    tab, cpu = ops.WeightTable(w, g, 0.01), ops.WeightTable(ref, rg, 0.01)
+    for step in range(1, 4):
+        ops.adam_step(tab)
+        ops.adam_step(cpu)
+        assert float(tab.hp[5]) == step and int(tab.hp.view(torch.int32)[7]) == 0
+    for a, b in zip(w, ref):
+        torch.testing.assert_close(a.cpu(), b, rtol=1e-4, atol=1e-6)
+
+
+def test_status_word_is_one_per_device():
+    assert ops.gemm_status("cuda") is ops.gemm_status(torch.device("cuda", torch.cuda.current_device()))
