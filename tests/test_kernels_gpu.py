@@ -614,3 +614,29 @@ def test_adam_advances_its_step_once_per_launch(shapes):
 
 def test_status_word_is_one_per_device():
     assert ops.gemm_status("cuda") is ops.gemm_status(torch.device("cuda", torch.cuda.current_device()))
+
+
+@pytest.mark.parametrize("width", [48, 100, 256, 300])
+def test_spmm_dense_tiles_do_not_depend_on_the_depth_of_the_ring(tiles_on_small_matrices, width):
+    """The rule that deepens the ring for chain-bound matrices changes no sum: every depth gives the same bits."""
+    g = _dense_corner_graph()
+    x = _rand2d(g.num_vertices, width, 1)
+    csr = build_normalized_csr(g).to(DEV)
+    tp = ops.api.tile_plan(csr)
+    results = []
+    for stages in (2, 3, 4, 6):
+        ops.api.set_aggregation_tiles(stages=stages)
+        out = ops.alloc2d(g.num_vertices, width, DEV)
+        ops.spmm(csr, x, out)
+        results.append(out)
+    for r in results[1:]:
+        assert torch.equal(r, results[0])
+    # both sides of the rule
+    ops.api.set_aggregation_tiles(stages=2)
+    longest, tiles = tp.longest_unit, tp.num_tiles
+    tp.longest_unit = tiles // 148 + 1
+    assert tp.ring_stages(256, 2) == 4 and tp.ring_stages(64, 2) == 2 and tp.ring_stages(256, 3) == 3
+    tp.longest_unit = max(1, tiles // 148)
+    assert tp.ring_stages(256, 2) == 2 or tiles < 148
+    tp.longest_unit = longest
+    _status_ok()
