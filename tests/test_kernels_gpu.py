@@ -640,3 +640,38 @@ def test_spmm_dense_tiles_do_not_depend_on_the_depth_of_the_ring(tiles_on_small_
     assert tp.ring_stages(256, 2) == 2 or tiles < 148
     tp.longest_unit = longest
     _status_ok()
+
+
+def test_workspaces_of_streams_and_of_a_callers_recording():
+    """Products that need a workspace, on two streams at once and in a CUDA graph recorded by the caller: a workspace belongs to
+    one stream, and one that a recording asks for belongs to that recording (its memory is not handed to later calls)."""
+    n, k, m = 20_000, 64, 48
+    x, dy = [_rand2d(n, k, s) for s in (1, 2)], [_rand2d(n, m, s) for s in (3, 4)]
+    dw = [ops.alloc2d(k, m, DEV) for _ in range(2)]
+    ref = []
+    for i in range(2):
+        ops.gemm(x[i], dy[i], dw[i], trans_a=True, precision="fp32")
+        ref.append(dw[i].clone())
+    dev = x[0].device
+    names = {}
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for rep in range(20):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                ops.gemm(x[i], dy[i], dw[i], trans_a=True, precision="fp32")
+                names[i] = ops.api._scratch_buf(dev, "splitk", 1).data_ptr()
+        torch.cuda.synchronize()
+        assert names[0] != names[1]
+        assert torch.equal(dw[0], ref[0]) and torch.equal(dw[1], ref[1])
+    g = torch.cuda.CUDAGraph()
+    kept = set(ops.api._workspaces.pool)
+    with torch.cuda.graph(g):
+        ops.gemm(x[0], dy[0], dw[0], trans_a=True, precision="fp32")
+    assert set(ops.api._workspaces.pool) == kept
+    ops.gemm(x[1], dy[1], dw[1], trans_a=True, precision="fp32")         # eager calls in between leave the recording alone
+    ops.api._scratch_buf(dev, "splitk", 1 << 24).fill_(7.0)
+    dw[0].zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(dw[0], ref[0])
