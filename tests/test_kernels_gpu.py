@@ -62,9 +62,11 @@ def _dense_corner_graph(seed=5):
     return rmat(6000, 600000, a=0.6, b=0.17, c=0.17, seed=seed)
 
 
-def test_spmm_dense_tiles_are_exact_on_integer_data(tiles_on_small_matrices):
+@pytest.mark.parametrize("stages", [None, 2])
+def test_spmm_dense_tiles_are_exact_on_integer_data(tiles_on_small_matrices, stages):
     """Structure check without a tolerance: unit edge values and small integer features are exact in TF32, so the
-    tensor-core tiles plus the residual gather must reproduce the fp32 product bit for bit."""
+    tensor-core tiles plus the residual gather must reproduce the fp32 product bit for bit.  The rule gives matrices of test size the deep ring; large ones run two stages."""
+    ops.api.set_aggregation_tiles(stages=stages)
     g = _dense_corner_graph()
     a = build_normalized_csr(g)
     a.val = torch.ones_like(a.val)
@@ -85,8 +87,10 @@ def test_spmm_dense_tiles_are_exact_on_integer_data(tiles_on_small_matrices):
     _status_ok()
 
 
+@pytest.mark.parametrize("stages", [None, 2])
 @pytest.mark.parametrize("width", [48, 128, 256])
-def test_spmm_dense_tiles_match_oracle_relu_accumulate(tiles_on_small_matrices, width):
+def test_spmm_dense_tiles_match_oracle_relu_accumulate(tiles_on_small_matrices, width, stages):
+    ops.api.set_aggregation_tiles(stages=stages)
     g = _dense_corner_graph(seed=6)
     a = build_normalized_csr(g)
     ad = a.to(DEV)
@@ -617,28 +621,34 @@ def test_status_word_is_one_per_device():
 
 
 @pytest.mark.parametrize("width", [48, 100, 256, 300])
-def test_spmm_dense_tiles_do_not_depend_on_the_depth_of_the_ring(tiles_on_small_matrices, width):
-    """The rule that deepens the ring for chain-bound matrices changes no sum: every depth gives the same bits."""
+def test_spmm_dense_tiles_do_not_depend_on_the_depth_of_the_ring(tiles_on_small_matrices, width, monkeypatch):
+    """The depth of the tile kernel's ring changes no sum: every depth gives the same bits, and the one that was asked for is
+    the one that runs (the kernel lowers it only to what fits 200 KB)."""
     g = _dense_corner_graph()
     x = _rand2d(g.num_vertices, width, 1)
     csr = build_normalized_csr(g).to(DEV)
     tp = ops.api.tile_plan(csr)
+    run, passed = ops.api._k().mk_spmm_tiles, []
+
+    class Spy:
+        def __getattr__(self, name):
+            return getattr(native, name)
+
+        def mk_spmm_tiles(self, *args):
+            passed.append(args[19])
+            return run(*args)
+
+    native = ops.api._k()
+    monkeypatch.setattr(ops.api, "_k", lambda spy=Spy(): spy)
     results = []
-    for stages in (2, 3, 4, 6):
+    for stages in (None, 2, 3, 4, 6):
         ops.api.set_aggregation_tiles(stages=stages)
         out = ops.alloc2d(g.num_vertices, width, DEV)
         ops.spmm(csr, x, out)
         results.append(out)
+    assert passed == [tp.ring_stages(ops.api.pad_cols(width, 4)), 2, 3, 4, 6]
     for r in results[1:]:
         assert torch.equal(r, results[0])
-    # both sides of the rule
-    ops.api.set_aggregation_tiles(stages=2)
-    longest, tiles = tp.longest_unit, tp.num_tiles
-    tp.longest_unit = tiles // 148 + 1
-    assert tp.ring_stages(256, 2) == 4 and tp.ring_stages(64, 2) == 2 and tp.ring_stages(256, 3) == 3
-    tp.longest_unit = max(1, tiles // 148)
-    assert tp.ring_stages(256, 2) == 2 or tiles < 148
-    tp.longest_unit = longest
     _status_ok()
 
 
