@@ -601,6 +601,22 @@ def test_gemm_fp32_weight_gradient_split_reduction(n, k, m):
         assert k == 1 or float(dw.as_strided((k, ld), (ld, 1))[:, m:].abs().sum()) == 0.0
 
 
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("n,k,m", [(1000, 33, 5), (12803, 105, 51), (3000, 200, 201)])
+def test_gemm_fp32_weight_gradient_into_columns_of_a_wider_matrix(n, k, m, accumulate):
+    """The result is the first columns of a matrix whose other columns belong to somebody else: they keep their values, in both
+    kernels that add the parts up (few and many elements).  At most one fp32 rounding per term and per part."""
+    assert n * k * m < 1 << 27 and ops.api._simt_splits(k, m, n) > 1
+    x, dy = _rand2d(n, k, 1), _rand2d(n, m, 2)
+    wide = torch.full((k, (m + 16) // 8 * 8), 3.0, device=DEV)
+    ops.gemm(x, dy, wide[:, :m], trans_a=True, accumulate=accumulate, precision="fp32")
+    X, DY = x.cpu().double(), dy.cpu().double()
+    ref, base = X.t() @ DY, 3.0 if accumulate else 0.0
+    bound = (n + 300) * 2.0 ** -24 * (X.abs().t() @ DY.abs() + base)
+    assert bool(((wide[:, :m].cpu().double() - ref - base).abs() <= bound).all())
+    assert bool((wide[:, m:] == 3.0).all())
+
+
 @pytest.mark.parametrize("shapes", [[(1, 4)], [(16, 64)], [(602, 256), (256, 41), (7, 3)], [(2400, 512)]])
 def test_adam_advances_its_step_once_per_launch(shapes):
     """One block, several, and more work than the grid has threads: the step counter moves by one per launch and the ticket
