@@ -84,6 +84,17 @@ def test_engine_refuses_an_epoch_whose_kernels_reported_an_expired_wait():
     e.read_metrics()
 
 
+def test_metrics_need_no_allocation_of_their_own():
+    """The page-locked words of the metrics are there when the engine is prepared; reading metrics only copies into them."""
+    g = erdos_renyi(500, 6, seed=6)
+    e, _ = run_single(GCN(2, 16, 5, 32), g, synthetic_dataset(g, 32, 5, seed=7), 0, device="cuda")
+    block = e._pinned
+    assert block is not None and block[0].is_pinned() and block[1].is_pinned()
+    e.run_epoch(0)
+    m = e.read_metrics()
+    assert e._pinned is block and m["loss"] == float(block[0][0]) / 500 and int(block[1]) == 0
+
+
 def test_cuda_graph_replay_equals_eager():
     g = erdos_renyi(2000, 10, seed=6)
     d = synthetic_dataset(g, 32, 5, seed=7)
