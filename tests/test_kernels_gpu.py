@@ -183,6 +183,43 @@ def test_gemm_grad_weight_split_reduction(n, k, m):
     _status_ok()
 
 
+@pytest.mark.parametrize("n", [64, 128, 129, 1000, 1024, 1025])
+def test_short_weight_gradients_eager_and_recorded(n):
+    """Reductions on both sides of the lines of the split rule: a recorded product is split from 129 rows on, an eager one, whose
+    second launch costs host time, from 1,025 on; both are the same sum (TF32: 10 mantissa bits per factor)."""
+    k, m = 130, 41
+    x, dy, out = _rand2d(n, k, 1), _rand2d(n, m, 2), ops.alloc2d(k, m, DEV)
+    ref = x.cpu().double().t() @ dy.cpu().double()
+    bound = 2.0 ** -9 * (x.cpu().double().abs().t() @ dy.cpu().double().abs())
+
+    def launches(f):
+        before = ops.api.launch_count
+        f()
+        return ops.api.launch_count - before
+
+    def check():
+        assert bool(((out.cpu().double() - ref).abs() <= bound).all())
+        out.zero_()
+
+    assert launches(lambda: ops.gemm(x, dy, out, trans_a=True)) == (1 if n <= 1024 else 2)
+    check()
+    g, held = torch.cuda.CUDAGraph(), {}
+    with ops.api.recording_scratch(held):
+        assert launches(lambda: ops.gemm(x, dy, out, trans_a=True)) == (1 if n <= 128 else 2)
+        check()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g):
+            assert launches(lambda: ops.gemm(x, dy, out, trans_a=True)) == (1 if n <= 128 else 2)
+    g.replay()
+    check()
+    own = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(own):                      # recorded by the caller
+        assert launches(lambda: ops.gemm(x, dy, out, trans_a=True)) == (1 if n <= 128 else 2)
+    own.replay()
+    check()
+    _status_ok()
+
+
 @pytest.mark.parametrize("n,k,m", [(40000, 256, 256), (33001, 256, 41), (70000, 100, 128), (20000, 64, 200)])
 def test_gemm_row_streaming_kernel(n, k, m):
     """The persistent short-reduction GEMM (weights resident in shared memory, rows streamed, two accumulators in tensor
