@@ -316,3 +316,31 @@ def test_fusions_and_shared_gradients_on_random_graphs(seed, dropout):
         if x is None and y is None:
             continue                    # a weight whose product nobody reads
         assert float((x - y).abs().max()) <= 3 * 100 * 6e-8 * max(1.0, float(y.abs().max())), seed
+
+
+class _StaticNet(AbstractApplication):
+    """Aggregated products of the input that meet again: one of them feeds a product directly, and a dropout of another branch
+    stands between a product and its aggregation."""
+
+    def __init__(self, dropout):
+        super().__init__(16)
+        self.dropout_p = dropout
+
+    def forward(self, input):  # noqa: A002
+        m = self.fc(input, 8)
+        h = self.relu(self.fc(input, 8))
+        if self.dropout_p:
+            h = self.dropout(h, self.dropout_p)
+        t = self.fc(self.aggregation(m, NORM_SUM), 8)               # product of a hoisted aggregation's output
+        return self.softmax(self.fc(self.add(t, h), 4))
+
+
+def test_static_inputs_follow_a_product_behind_a_hoisted_aggregation():
+    """The rewritten graph computes the same map: fp32 curves that differ by the order of a few additions."""
+    g = rmat(60, 400, seed=5)
+    d = synthetic_dataset(g, 16, 4, seed=6)
+    plain, _ = run_single(_StaticNet(0.0), g, d, 4, optimizer=SGDOptimizer(0.05))
+    fast, _ = run_single(_StaticNet(0.0), g, d, 4, optimizer=SGDOptimizer(0.05), static_inputs=True)
+    assert len(fast.prog.invariant_ops) > 1
+    for a, b in zip(plain.history, fast.history):
+        assert abs(a["loss"] - b["loss"]) <= 1e-5 * max(1.0, abs(a["loss"]))
