@@ -335,12 +335,14 @@ class _StaticNet(AbstractApplication):
         return self.softmax(self.fc(self.add(t, h), 4))
 
 
-def test_static_inputs_follow_a_product_behind_a_hoisted_aggregation():
-    """The rewritten graph computes the same map: fp32 curves that differ by the order of a few additions."""
+@pytest.mark.parametrize("dropout", [0.0, 0.4])
+def test_static_inputs_follow_a_product_behind_a_hoisted_aggregation(dropout):
+    """The rewritten graph computes the same map, with the same dropout masks: fp32 curves that differ by the order of a few
+    additions."""
     g = rmat(60, 400, seed=5)
     d = synthetic_dataset(g, 16, 4, seed=6)
-    plain, _ = run_single(_StaticNet(0.0), g, d, 4, optimizer=SGDOptimizer(0.05))
-    fast, _ = run_single(_StaticNet(0.0), g, d, 4, optimizer=SGDOptimizer(0.05), static_inputs=True)
+    plain, _ = run_single(_StaticNet(dropout), g, d, 4, optimizer=SGDOptimizer(0.05))
+    fast, _ = run_single(_StaticNet(dropout), g, d, 4, optimizer=SGDOptimizer(0.05), static_inputs=True)
     assert len(fast.prog.invariant_ops) == 1
     for a, b in zip(plain.history, fast.history):
         assert abs(a["loss"] - b["loss"]) <= 1e-5 * max(1.0, abs(a["loss"]))
