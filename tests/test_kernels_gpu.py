@@ -762,3 +762,59 @@ def test_spmm_at_fp32_precision_keeps_off_the_tiles(tiles_on_small_matrices, mon
     ops.spmm(csr, x, again)
     assert torch.equal(again, tf32)
     _status_ok()
+
+
+def _random_block(rows, cols, seed):
+    """Rows of every length from none to several batches, one of them cut into items."""
+    g = torch.Generator().manual_seed(seed)
+    deg = torch.randint(0, 50, (rows,), generator=g)
+    deg[torch.randint(0, rows, (max(1, rows // 10),), generator=g)] = 0
+    deg[rows // 2] = 1500
+    rowptr = torch.zeros(rows + 1, dtype=torch.int64)
+    rowptr[1:] = torch.cumsum(deg, 0)
+    nnz = int(rowptr[-1])
+    csr = NormalizedCSR(rowptr, torch.randint(0, cols, (nnz,), generator=g).to(torch.int32), torch.randn(nnz, generator=g), rows, cols)
+    return csr, torch.repeat_interleave(torch.arange(rows), deg), deg.double()[:, None]
+
+
+@pytest.mark.parametrize("rows", [6, 9001])
+@pytest.mark.parametrize("width", [4, 16, 17, 32, 33, 48, 64, 65, 96, 97, 128, 129, 256, 257, 512, 640, 1000])
+def test_spmm_halo_and_push_forms_with_two_buffers_as_ranks(rows, width):
+    """The forms of the gather that reach other ranks, with two buffers of this GPU in the ranks' places: columns behind the local
+    ones are read from their owner's buffer, and the rows of a pushed block are added into theirs (in no fixed order).  Against
+    float64: one rounding per product and per addition."""
+    import ctypes as C
+    from types import SimpleNamespace
+    n_local, slots, owned = 300, 211, 400
+    csr, of_row, deg = _random_block(rows, n_local + slots, rows)
+    ranks = [_rand2d(owned, width, s) for s in (1, 2)]
+    g = torch.Generator().manual_seed(3)
+    mirror = torch.stack([torch.randint(0, 2, (slots,), generator=g), torch.randint(0, owned, (slots,), generator=g)], 1).to(torch.int32)
+    ptrs = (C.c_void_p * 2)(*[t.data_ptr() for t in ranks])
+    host = [t.cpu().double() for t in ranks]
+    operand = torch.cat([host[0][:n_local], torch.stack(host)[mirror[:, 0].long(), mirror[:, 1].long()]])
+    val, col = csr.val.double()[:, None], csr.col.long()
+
+    def product(op, v):
+        return torch.zeros(rows, op.shape[1], dtype=torch.float64).index_add_(0, of_row, op[col] * v)
+
+    dev, out = csr.to(DEV), _rand2d(rows, width, 4)
+    halo = SimpleNamespace(n_local=n_local, mirror=mirror.to(DEV), peer_ptrs=ptrs, num_peers=2)
+    ops.spmm(dev, ranks[0], out, relu=True, halo=halo)
+    ref, bound = product(operand, val), 2.0 ** -24 * (deg + 3) * product(operand.abs(), val.abs())
+    assert bool(((out.cpu().double() - torch.relu(ref)).abs() <= bound).all())
+    # push: row r of the block goes to row target[r, 1] of buffer target[r, 0]; several rows may meet in one
+    x = _rand2d(n_local + slots, width, 5)
+    target = torch.stack([torch.randint(0, 2, (rows,), generator=g), torch.randint(0, owned, (rows,), generator=g)], 1).to(torch.int32)
+    ops.spmm_push(dev, x, ops.api._ld(ranks[0]), target.to(DEV), ptrs, 2)
+    xs = x.cpu().double()
+    part, mass = product(xs, val), product(xs.abs(), val.abs())
+    for r in range(2):
+        mine = target[:, 0] == r
+        to = target[mine, 1].long()
+        want = host[r].clone().index_add_(0, to, part[mine])
+        terms = torch.zeros(owned, 1, dtype=torch.float64).index_add_(0, to, deg[mine] + 2)
+        total = host[r].abs().index_add_(0, to, mass[mine])
+        assert bool(((ranks[r].cpu().double() - want).abs() <= 2.0 ** -24 * (terms + 2) * total).all())
+        ld = ops.api._ld(ranks[r])
+        assert float(ranks[r].as_strided((owned, ld), (ld, 1))[:, width:].abs().sum()) == 0.0
